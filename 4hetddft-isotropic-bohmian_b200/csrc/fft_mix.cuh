@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(MixPipe<M, C2, pipe_z_regs<M, C2>()>::threads,
 // energies' rounding was 1.3 to 1.8 times that of the summed fields.
 // ---------------------------------------------------------------------------
 struct MixZEnergyArgs {
-  int npid, nxh, nx, nz;
+  int npid, nxh, nx, nz, w;  // w: pencils per CTA
   long sf;
   const double2 *ta;
   const BoxPair *box;
@@ -555,7 +555,9 @@ __global__ void __launch_bounds__(M::kMaxThreads) k_mix_zenergy(MixZEnergyArgs a
   extern __shared__ __align__(16) unsigned char smem_raw[];
   after_previous();
   __shared__ double sh[32];
-  const int W = blockDim.x / M::T;
+  // the CTA is rounded up to whole warps (block_sum); the threads past W T, whose
+  // t is T or more, take neither step and add zeros
+  const int W = a.w, VP = W * M::T;
   const int w = threadIdx.x % W, t = threadIdx.x / W;
   C2 *S0 = reinterpret_cast<C2 *>(smem_raw), *S = S0 + w * M::PP;
   C2 *V = S0 + W * M::PP + threadIdx.x;  // F at cells of this thread only
@@ -581,7 +583,7 @@ __global__ void __launch_bounds__(M::kMaxThreads) k_mix_zenergy(MixZEnergyArgs a
     for (int e = 0; e < M::E; e++) {
       const double x = v[e].x, y = v[e].y;
       e1 += (x * x + y * y) * __ldg(a.k1 + pid + (long)M::k(t, e) * a.sf);
-      V[e * blockDim.x] = v[e];
+      V[e * VP] = v[e];
     }
   }
   __syncthreads();
@@ -605,7 +607,7 @@ __global__ void __launch_bounds__(M::kMaxThreads) k_mix_zenergy(MixZEnergyArgs a
     mix_fwd2<M, false>(v, S, t);
 #pragma unroll
     for (int e = 0; e < M::E; e++) {
-      const C2 F = V[e * blockDim.x];
+      const C2 F = V[e * VP];
       e2 += (F.x * v[e].x + F.y * v[e].y) * __ldg(a.k2 + pid + (long)M::k(t, e) * a.sf);
     }
   }
@@ -879,12 +881,13 @@ struct MixLaunch {
   }
   static int zenergy(Handle *h, MixZEnergyArgs &a, bool f32, int w, int *ctas) {
     if constexpr (sizeof(C2) == 16) {
-      w = capv(w);
+      a.w = w = capv(w);
       *ctas = (a.npid + w - 1) / w;
+      const int threads = (w * M::T + 31) / 32 * 32;  // at most kMaxThreads, as w T is
       if (!f32) {
-        HE4_TRY(launch_after(h, *ctas, w * M::T, smem_v(w), k_mix_zenergy<M, double2>, a));
+        HE4_TRY(launch_after(h, *ctas, threads, smem_v(w), k_mix_zenergy<M, double2>, a));
       } else if constexpr (kPow2) {
-        HE4_TRY(launch_after(h, *ctas, w * M::T, smem_v(w), k_mix_zenergy<M, float2>, a));
+        HE4_TRY(launch_after(h, *ctas, threads, smem_v(w), k_mix_zenergy<M, float2>, a));
       }
       HE4_LAUNCHED(h);
       return HE4_OK;

@@ -8,8 +8,9 @@
 
 namespace he4 {
 
-// Sum of v over the block; the result is valid in thread 0.
-// `sh` must hold blockDim/32 doubles.
+// Sum of v over the block; the result is valid in thread 0.  The block is of
+// whole warps (a multiple of 32 threads: every lane that a shuffle names is
+// there), and `sh` holds one double per warp.
 __device__ __forceinline__ double block_sum(double v, double *sh) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nthreads = blockDim.x * blockDim.y * blockDim.z;
