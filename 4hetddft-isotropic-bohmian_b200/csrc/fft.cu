@@ -767,6 +767,13 @@ int fft_r2c(Handle *h, int n, const double *const *in, double2 *const *out) {
   return HE4_OK;
 }
 
+// The x pass writes the row pairs that touch the impurity box's planes, the y pass
+// transforms the planes of the force box, one more on either side.  Those two stay
+// exact zeros through any number of in-place transforms: with odd ny the row that a
+// pair shares with a plane beyond the box is the first or last of its plane, the
+// row beside it in the pair is the last or first of the box's plane, and both are
+// zero in `in`, since a box that comes within 2 m cells of a face in y is the whole
+// grid (k_box_find).  A pair of zero rows transforms to zeros.
 int fft_r2c_box(Handle *h, const double *in, double2 *out) {
   const FftPlan &P = h->fft;
   const double *ri[1] = {in};
