@@ -437,6 +437,9 @@ int field_all(Handle *h, bool split = false);
 // after a merged evaluation: compute the named intermediate fields of the
 // same state without touching pot4
 int field_split_fields(Handle *h);
+// after a merged evaluation with float grids: the gradients of den and the
+// alpha_s integrals in the FP64 grids dxden.. and intx..
+int field_alpha_fp64(Handle *h);
 // impurity.cu: denx, psix, hpsix on the particle box; quantum force term;
 // reset of the box to the whole grid
 int impurity_density(Handle *h);

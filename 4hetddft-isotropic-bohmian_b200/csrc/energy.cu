@@ -4,10 +4,12 @@
 // summed in k space from the x/y spectra that every evaluation keeps
 // (k_mix_zenergy), so a merged evaluation's missing delj4 and uimp are not
 // computed for them; k_energy evaluates the first derivatives of psi and the
-// other grid sums per CTA.  A single CTA then adds the per-CTA partials in
-// index order, and the host combines the sums with the formulas of
-// energy.f90:374-407.  256^3: split evaluation and one sum kernel 5.6 ms (FP64)
-// and 3.8 ms (FP32 form) per call before, 0.88 and 0.86 ms here.
+// other grid sums per CTA.  Up to 32 CTAs then add the per-CTA partials in a fixed
+// order, and the host combines the sums with the formulas of energy.f90:374-407.
+// The gradients and alpha_s integrals of ealphas are FP64 grids in both forms
+// (field_alpha_fp64).  256^3, per call: split evaluation and one sum kernel 4.9 ms
+// (FP64) and 3.8 ms (FP32 form) before, 1.0 and 1.7 here (0.7 of the latter for
+// those grids).
 #include <algorithm>
 
 #include "common.cuh"
@@ -23,17 +25,17 @@ struct EArgs {
 
 constexpr int kESums = 7;  // ekin4, ecor4, ealphas, esolid, ekinqx, elj4, eHeX
 
-// T: the type of the evaluation's intermediate grids (dencg, the gradients, the
-// alpha_s integrals).  HV: i0..i2 hold falfs * int_i (the float merged
-// evaluation writes the products over the integrals).  CONV: elj4 and eHeX
-// from delj4 and uimp (z lengths without the k-space form).
-template <typename T, bool HV, bool CONV>
+// T: the type of the evaluation's dencg and denalf (float: results of FP32
+// transforms, which a wider grid would hold unchanged).  CONV: elj4 and eHeX from
+// delj4 and uimp (z lengths without the k-space form).
+template <typename T, bool CONV>
 __global__ void k_energy(const double2 *__restrict__ psi, const double *__restrict__ den, const T *__restrict__ dencg,
-                         const T *__restrict__ denalf, const T *__restrict__ dx, const T *__restrict__ dy,
-                         const T *__restrict__ dz, const T *__restrict__ i0, const T *__restrict__ i1,
-                         const T *__restrict__ i2, const double *__restrict__ psix, const double *__restrict__ hpsix,
-                         const double *__restrict__ delj4, const double *__restrict__ uimp,
-                         const BoxPair *__restrict__ bp, double *part, size_t stride, Stencil st, Geo g, EArgs a) {
+                         const T *__restrict__ denalf, const double *__restrict__ dx, const double *__restrict__ dy,
+                         const double *__restrict__ dz, const double *__restrict__ i0, const double *__restrict__ i1,
+                         const double *__restrict__ i2, const double *__restrict__ psix,
+                         const double *__restrict__ hpsix, const double *__restrict__ delj4,
+                         const double *__restrict__ uimp, const BoxPair *__restrict__ bp, double *part, size_t stride,
+                         Stencil st, Geo g, EArgs a) {
   __shared__ double sh[32];
   const int i = blockIdx.x * 32 + threadIdx.x;
   const int j = blockIdx.y * 8 + threadIdx.y;
@@ -47,10 +49,7 @@ __global__ void k_energy(const double2 *__restrict__ psi, const double *__restri
     v[0] = (d1.x * d1.x + d1.y * d1.y) + (d2.x * d2.x + d2.y * d2.y) + (d3.x * d3.x + d3.y * d3.y);
     const double dn = den[t], dc = (double)dencg[t];
     v[1] = dn * dc * dc * (a.aux1 + a.aux2 * dc);
-    if (a.otc) {
-      const double s = (double)dx[t] * (double)i0[t] + (double)dy[t] * (double)i1[t] + (double)dz[t] * (double)i2[t];
-      v[2] = HV ? s : (1.0 - (double)denalf[t] / a.den0s) * s;
-    }
+    if (a.otc) v[2] = (1.0 - (double)denalf[t] / a.den0s) * (dx[t] * i0[t] + dy[t] * i1[t] + dz[t] * i2[t]);
     v[3] = dn * (1.0 + tanh(a.beta * (dn - a.den_m)));
     const Box b = bp->cur;  // psix is zero outside the particle box
     if (b.full || (!b.empty && k >= b.lo[2] && k <= b.hi[2] && j >= b.lo[1] && j <= b.hi[1] && i >= b.lo[0] &&
@@ -97,17 +96,19 @@ int compute_energy(Handle *h, he4_energies *E) {
     set_error("reduction workspace too small");
     return HE4_E_STATE;
   }
-  auto grids = [&](auto kern, auto *dencg, auto *denalf, auto *dx, auto *dy, auto *dz, auto *i0, auto *i1, auto *i2) {
-    kern<<<gr, block3(), 0, h->stream>>>(h->psi, h->den, dencg, denalf, dx, dy, dz, i0, i1, i2, h->psix, h->hpsix,
-                                         h->delj4, h->uimp, h->box, h->red, nb, h->st, g, a);
+  auto grids = [&](auto kern, auto *dencg, auto *denalf) {
+    kern<<<gr, block3(), 0, h->stream>>>(h->psi, h->den, dencg, denalf, h->dxden, h->dyden, h->dzden, h->intx, h->inty,
+                                         h->intz, h->psix, h->hpsix, h->delj4, h->uimp, h->box, h->red, nb, h->st, g,
+                                         a);
   };
-  if (!kspace)
-    grids(k_energy<double, false, true>, h->dencg, h->denalf, h->dxden, h->dyden, h->dzden, h->intx, h->inty, h->intz);
-  else if (h->real32 && !h->split_valid)  // the float grids of the merged evaluation
-    grids(k_energy<float, true, false>, h->g32[0], h->g32[1], h->g32[2], h->g32[3], h->g32[4], h->g32[5], h->g32[6],
-          h->g32[7]);
-  else
-    grids(k_energy<double, false, false>, h->dencg, h->denalf, h->dxden, h->dyden, h->dzden, h->intx, h->inty, h->intz);
+  if (!kspace) {
+    grids(k_energy<double, true>, h->dencg, h->denalf);
+  } else if (h->real32 && !h->split_valid) {  // the float grids of the merged evaluation
+    if (a.otc) HE4_TRY(field_alpha_fp64(h));
+    grids(k_energy<float, false>, h->g32[0], h->g32[1]);
+  } else {
+    grids(k_energy<double, false>, h->dencg, h->denalf);
+  }
   HE4_LAUNCHED(h);
   if (kspace) {
     HE4_TRY(finalize_sums<5>(h, h->red, nb, (int)nb, 1.0, 1.0, h->scal + 16));

@@ -961,6 +961,27 @@ static int field_poten_merged_f32(Handle *h) {
   return branch(h, h->side, h->stream, h->ev[4]);
 }
 
+// What ealphas needs beside denalf, with the FP32-convolution form's real grids in
+// FP64 (field_poten_merged_f32 keeps the gradients and falfs * int_i as floats):
+// the alpha_s part of the split evaluation, its sources formed on load.
+int field_alpha_fp64(Handle *h) {
+  HE4_TRY(launch_grad(h));
+  HE4_TRY(widen(h, h->g32[1], h->denalf, h->N));
+  const void *in[3] = {h->dxden, h->dyden, h->dzden};
+  double2 *sp[3] = {h->spec[1], h->spec[2], h->spec[3]};
+  XLoad ld;
+  ld.op = XLOAD_ALFA;
+  ld.aux0 = h->denalf;
+  ld.c0 = 1.0 / h->p.den0s;
+  HE4_TRY(fft_r2c_load(h, 3, in, sp, ld));
+  ZOp ops[3] = {{h->spec[1], h->spec[1], h->kalfs, h->renor, -1},
+                {h->spec[2], h->spec[2], h->kalfs, h->renor, -1},
+                {h->spec[3], h->spec[3], h->kalfs, h->renor, -1}};
+  HE4_TRY(fft_z_conv(h, 3, ops));
+  double *out[3] = {h->intx, h->inty, h->intz};
+  return fft_c2r(h, 3, sp, out);
+}
+
 // pot4 of the FP32-convolution form's merged evaluation: lin (in g32[8]),
 // dencg (g32[0]) and h_i (g32[5..7]) are float grids, den and pot4 double
 int launch_pot4_merged_f32(Handle *h) {
