@@ -1009,6 +1009,11 @@ using namespace he4;
 using namespace he4::fno;
 
 namespace {
+// Dynamic shared memory limit of the k_contract kernels, one value for every size: a
+// limit of each call's own need can be lowered by another thread's call before this
+// one's launch, which then fails.  J K <= 6144 entries and the dispatch below need
+// 96 KB at most (J = 6144, K = 1: two entries per j).
+constexpr int kContractSmem = 96 * 1024;
 template <int KT, int JS>
 int launch_contract(const void *x, void *y, const float2 *A, unsigned ncol, int J, int K, unsigned inner, int in_real,
                     int out_real, int accumulate, cudaStream_t s) {
@@ -1018,7 +1023,7 @@ int launch_contract(const void *x, void *y, const float2 *A, unsigned ncol, int 
   auto run = [&](auto kern) {
     // J K has 6144 entries at most (48 KB); the rounded-up rows and the partial sums may need more
     if (sm > 48 * 1024 &&
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess)
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kContractSmem) != cudaSuccess)
       return launched();
     kern<<<grid, warps * kCols, sm, s>>>(x, y, A, ncol, J, K, inner, accumulate);
     return launched();
