@@ -5,6 +5,8 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
+#include <iterator>
 #include <new>
 
 #include "common.cuh"
@@ -202,7 +204,11 @@ static int create(const he4_params *pin, Handle *h) {
                         &h->intx, &h->inty, &h->intz, &h->dxden, &h->dyden, &h->dzden, &h->penalty,
                         &h->corr, &h->denx, &h->psix, &h->hpsix, &h->uimp, &h->fx, &h->fy, &h->fz,
                         &h->rtmp[0], &h->rtmp[1], &h->rtmp[2], &h->rtmp[3]};
-  for (double **f : rfields) HE4_TRY(dalloc(f, N));
+  // (three of them with the room of a half spectrum, 2 H >= N, for fspec)
+  double **sfields[] = {&h->delj4, &h->penalty, &h->corr};
+  for (double **f : rfields)
+    HE4_TRY(dalloc(f, std::find(std::begin(sfields), std::end(sfields), f) != std::end(sfields) ? 2 * H : N));
+  for (int i = 0; i < 3; i++) h->fspec[i] = reinterpret_cast<double2 *>(*sfields[i]);
   HE4_TRY(dalloc(&h->counts, N));
   HE4_TRY(dalloc(&h->box, 1));
   HE4_TRY(dalloc(&h->gred, 1));
@@ -216,7 +222,6 @@ static int create(const he4_params *pin, Handle *h) {
     HE4_CUDA_TRY(cudaMemcpy(h->gred, &g0, sizeof(GridRed), cudaMemcpyHostToDevice));
   }
   for (int i = 0; i < 6; i++) HE4_TRY(dalloc(&h->spec[i], H));
-  for (int i = 6; i < 9; i++) HE4_TRY(dalloc(&h->spec[i], h->fp32 ? (H + 1) / 2 : H));
   double **pfields[] = {&h->rimp, &h->vimp, &h->aimp, &h->rimpold[0], &h->rimpold[1], &h->rimpold[2],
                         &h->vimpold[0], &h->vimpold[1], &h->vimpold[2], &h->aimpold[0], &h->aimpold[1],
                         &h->qr, &h->qv, &h->pcr, &h->pcv};

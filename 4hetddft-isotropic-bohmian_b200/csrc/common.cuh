@@ -249,7 +249,10 @@ struct Handle {
   unsigned int *counts = nullptr;
   BoxPair *box = nullptr;  // device: support of denx/psix/hpsix
   // spectra work buffers [H] complex
-  double2 *spec[9] = {nullptr};  // float2 in the FP32-convolution form
+  double2 *spec[6] = {nullptr};  // float2 in the FP32-convolution form
+  // the forces' spectra of a merged evaluation, whose other branch has spec[1..3]:
+  // the room of delj4, penalty and corr, which every split evaluation writes anew
+  double2 *fspec[3] = {nullptr};
 
   // particles [3][npar]
   double *rimp = nullptr, *vimp = nullptr, *aimp = nullptr;
@@ -419,8 +422,9 @@ int field_potenimp(Handle *h, bool split);
 int field_poten(Handle *h, bool split, double *pot4);
 // full: the force field on the whole grid; otherwise only where the gather
 // reads it (a time step's need).  field_forces recomputes just the field.
-int field_forceimp(Handle *h, bool full);
-int field_forces(Handle *h, bool full);
+// merged: within a merged evaluation (the spectra in fspec, not spec[1..3]).
+int field_forceimp(Handle *h, bool full, bool merged = false);
+int field_forces(Handle *h, bool full, bool merged = false);
 // the stencil passes of an evaluation (also timed by he4_bench_kernel)
 int launch_grad(Handle *h);
 // the merged evaluation may keep float intermediate grids (Handle::real32)

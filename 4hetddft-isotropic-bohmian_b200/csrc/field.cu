@@ -863,7 +863,7 @@ static int field_poten_merged(Handle *h) {
   // side, beside the rest: the forces, which need the spectrum of den, the
   // impurity's box and (non-periodic stencils) the gradient
   if (!otc) HE4_TRY(branch(h, h->stream, h->side, h->ev[2]));
-  HE4_TRY(on_side(h, [&] { return field_forceimp(h, false); }));
+  HE4_TRY(on_side(h, [&] { return field_forceimp(h, false, true); }));
   HE4_TRY(fft_z_sum(h, otc ? 4 : 3, terms, h->spec[2]));
   {
     double2 *sp[1] = {h->spec[2]};
@@ -950,7 +950,7 @@ static int field_poten_merged_f32(Handle *h) {
   // side, beside the rest: the forces, which need the spectrum of den, the
   // impurity's box and (non-periodic stencils) the gradient
   if (!otc) HE4_TRY(branch(h, h->stream, h->side, h->ev[2]));
-  HE4_TRY(on_side(h, [&] { return field_forceimp(h, false); }));
+  HE4_TRY(on_side(h, [&] { return field_forceimp(h, false, true); }));
   HE4_TRY(fft_z_sum(h, otc ? 4 : 3, terms, h->spec[2]));
   {
     double2 *sp[1] = {h->spec[2]};
@@ -1094,25 +1094,25 @@ int field_poten(Handle *h, bool split, double *pot4) {
 // The force field f_i on the grid: the whole grid (full) or only the cells
 // the trilinear gather reads (the impurity box widened by one cell), which
 // is what a time step needs.
-int field_forces(Handle *h, bool full) {
+int field_forces(Handle *h, bool full, bool merged) {
   // f_i = -IFFT(FFT(d_i rho) Vq) * renor / m_X = IFFT(-renor/m_X Vq i D_i fden)
   // (potenimp.f90:42-50, with the 1/m_X of :67-69 folded in)
   const double c = -h->renor / h->mAg_u;
   const int bz = full ? 0 : 1;
-  double2 *sp[3] = {h->spec[6], h->spec[7], h->spec[8]};  // (1 to 3: the alpha term's, meanwhile)
+  double2 *const *sp = merged ? h->fspec : h->spec + 1;
   if (h->p.icon == 8) {
-    ZOp ops[3] = {{h->spec[0], h->spec[6], h->vq, c, 0, 0, bz},
-                  {h->spec[0], h->spec[7], h->vq, c, 1, 0, bz},
-                  {h->spec[0], h->spec[8], h->vq, c, 2, 0, bz}};
+    ZOp ops[3] = {{h->spec[0], sp[0], h->vq, c, 0, 0, bz},
+                  {h->spec[0], sp[1], h->vq, c, 1, 0, bz},
+                  {h->spec[0], sp[2], h->vq, c, 2, 0, bz}};
     HE4_TRY(fft_z_conv(h, 3, ops));
   } else {
     // non-periodic stencils: FFT(d_i rho) is no multiple of FFT(rho), so the
     // gradients of this evaluation are transformed as the reference does
     const double *in[3] = {h->dxden, h->dyden, h->dzden};
     HE4_TRY(fft_r2c(h, 3, in, sp));
-    ZOp ops[3] = {{h->spec[6], h->spec[6], h->vq, c, -1, 0, bz},
-                  {h->spec[7], h->spec[7], h->vq, c, -1, 0, bz},
-                  {h->spec[8], h->spec[8], h->vq, c, -1, 0, bz}};
+    ZOp ops[3] = {{sp[0], sp[0], h->vq, c, -1, 0, bz},
+                  {sp[1], sp[1], h->vq, c, -1, 0, bz},
+                  {sp[2], sp[2], h->vq, c, -1, 0, bz}};
     HE4_TRY(fft_z_conv(h, 3, ops));
   }
   double *out[3] = {h->fx, h->fy, h->fz};
@@ -1126,8 +1126,8 @@ int field_forces(Handle *h, bool full) {
   return HE4_OK;
 }
 
-int field_forceimp(Handle *h, bool full) {
-  HE4_TRY(field_forces(h, full));
+int field_forceimp(Handle *h, bool full, bool merged) {
+  HE4_TRY(field_forces(h, full, merged));
   GatherArgs a;
   a.nx = h->nx;
   a.ny = h->ny;
