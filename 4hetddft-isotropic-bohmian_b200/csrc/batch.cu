@@ -63,8 +63,8 @@ static int apply_tiles(Handle *h, const int *t) {
 }
 
 // Coordinate search over the tile shapes of the three axes: for each axis
-// the candidates are the register-path splits N = N1 * N2 or, on the generic
-// path, 8..32 pencils per CTA; each candidate is timed as `reps` mean-field
+// the candidates are the two-step splits N = N1 * N2 (powers of two from 16 to 256)
+// or, for other lengths, 8..32 pencils per CTA; each candidate is timed as `reps` mean-field
 // evaluations of the handle's current state with CUDA events, the fastest
 // is kept before the next axis is searched.
 static int tune(Handle *h, int reps, double *best_ms, int *best) {

@@ -108,9 +108,11 @@ struct AxisPlan {
 struct FftPlan {
   int nx = 0, ny = 0, nz = 0, nxh = 0;
   AxisPlan ax, ay, az;
-  int wy = 8, wz = 8;   // pencils per CTA in the y and z passes (generic path)
-  int px = 8;           // complex pencils (= row pairs) per CTA in the x pass (generic path)
-  int n1[3] = {0, 0, 0};  // four-step split N = N1 * N2 per axis (register path)
+  // axis lengths other than the powers of two from 16 to 256: pencils per CTA in the
+  // y and z passes, complex pencils (row pairs) per CTA in the x pass
+  int wy = 8, wz = 8;
+  int px = 8;
+  int n1[3] = {0, 0, 0};  // those powers of two: first factor of N = N1 * N2 per axis
 };
 
 int fft_plan_init(FftPlan &P, int nx, int ny, int nz);
@@ -316,7 +318,11 @@ struct Handle {
 // that the other branch's kernels need and each block of a long grid pays for the
 // wait: 128^3 in FP32 10.6 -> 10.9 ms, 256^3 in FP32 44 -> 50 ms.  For the same
 // reason the side branch's kernels and the members of larger ensembles, which
-// share the GPU, start in the ordinary way.
+// share the GPU, start in the ordinary way.  A captured step costs more with
+// programmatic edges: 0.47 instead of 0.27 ms to instantiate and 0.44 instead of
+// 0.20 to destroy (0.15 and 0.09 without the side branch), so that they pay from
+// some 25 replays of a graph on (64^3: a fresh handle's first 13 steps, ten captures
+// among them, 6.3 ms, repeated ones 3.5).
 constexpr size_t kAfterPoints = 1 << 20;
 template <typename... P, typename... A>
 int launch_after(Handle *h, dim3 grid, dim3 block, size_t smem, void (*kern)(P...), A... args) {
@@ -370,7 +376,7 @@ struct ZOp {
 };
 int fft_z_conv(Handle *h, int n, const ZOp *ops);
 // z pass of a sum of convolutions: out = IFFT_z(sum_j coef_j K_j FFT_z(in_j))
-// (register-path z lengths only; at most 4 terms)
+// (two-step z lengths only; at most 4 terms)
 struct ZTerm {
   const double2 *in;
   const double *kern;
@@ -414,10 +420,13 @@ int setup_kernels(Handle *h);
 int narrow(Handle *h, const double *in, float *out, size_t n);
 int widen(Handle *h, const float *in, double *out, size_t n);
 
-// split: also write the named intermediate fields (uimp; delj4, corr,
-// ualphas, penalty) the way the reference's routines do; otherwise (the time
-// step path) the linear convolutions entering pot4 share one inverse FFT.
-// pot4: where the split poten writes its pot4.
+// split: the reference's three routines potenimp, poten and forceimp one after the
+// other, with the named intermediate fields (uimp; delj4, corr, ualphas, penalty);
+// pot4: where the split poten writes its pot4.  field_poten(split = false) is the
+// whole merged evaluation of the time step, the impurity chain (potenimp) and the
+// forces included: the linear convolutions entering pot4 share one inverse FFT, and
+// the branches interleave.  (An impurity chain of its own beside it would advance
+// the box twice and lose the previous support that has to be cleared.)
 int field_potenimp(Handle *h, bool split);
 int field_poten(Handle *h, bool split, double *pot4);
 // full: the force field on the whole grid; otherwise only where the gather

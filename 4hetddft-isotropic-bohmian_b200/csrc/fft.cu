@@ -11,9 +11,13 @@
 //   y pass  (complex), and
 //   z pass  (complex) fused with the k-space kernel multiply and the inverse
 //           z transform: FFT_z -> coef*K(k) (*i*D(k)) -> IFFT_z in one launch.
-// Each CTA stages a tile of pencils in shared memory and runs a mixed-radix
-// (2/3/4/5) Stockham transform between two shared buffers; pencils of one
-// tile are contiguous in x so every global access is a coalesced segment.
+// Axis lengths 36..250 with factors 2, 3 and 5 and the powers of two from 16 to 256
+// run as the two-step register passes of fft_mix.cuh (FP32 spectra: the powers of two
+// only), chosen per axis; this file holds their tables and launches.  The other
+// lengths (8..30) run the generic kernels below: each CTA stages a tile of pencils
+// in shared memory and runs a mixed-radix (2/3/4/5) Stockham transform between two
+// shared buffers; pencils of one tile are contiguous in x, so every global access is
+// a coalesced segment.
 #include <math.h>
 #include <stdlib.h>
 
@@ -527,9 +531,9 @@ int fft_plan_init(FftPlan &P, int nx, int ny, int nz) {
   return HE4_OK;
 }
 
-// Tile shapes: t = {n1 x, n1 y, n1 z, px, wy, wz}.  n1 applies to register
-// path axes (0 = default split), px / wy / wz (pencils per CTA, multiples of
-// 8 in [8, 32]) to generic-path axes; entries for the other path are ignored.
+// Tile shapes: t = {n1 x, n1 y, n1 z, px, wy, wz}.  n1 applies to the axes of 16 to
+// 256 points that are powers of two (0 = default split), px / wy / wz (pencils per
+// CTA, multiples of 8 in [8, 32]) to all others; an axis ignores the other entry.
 int fft_set_tiles(FftPlan &P, const int *t) {
   const int ns[3] = {P.nx, P.ny, P.nz};
   int n1[3];
@@ -712,7 +716,7 @@ static int yz_mix(Handle *h, int nb, double2 *const *buf, int axis, bool inverse
 }
 
 // in-place complex transform of every pencil along y (axis 1) or z (axis 2);
-// box (y pass, register path): only pencils whose z lies in the force box
+// box (y pass, two-step lengths): only pencils whose z lies in the force box
 static int strided_pass(Handle *h, int n, double2 *const *buf, int axis, bool inverse,
                         const BoxPair *box = nullptr) {
   const FftPlan &P = h->fft;

@@ -121,7 +121,7 @@ template <typename M, typename C2>
 constexpr int pipe_z_regs() { return 52 + (int)sizeof(C2) / 8 * M::E; }
 
 // twiddles w_N^(j1 k2) in both lane orders: ta[k2 N1 + j1], tb[j1 N2 + k2]
-// (AxisPlan::mixa / mixb), read through the cache with consecutive lanes on
+// (AxisPlan::mix: ta, then tb), read through the cache with consecutive lanes on
 // consecutive entries (x passes) or on one entry (y and z passes)
 
 // forward, first step: a[j2] = x[t + N1 j2] -> shared memory

@@ -6,18 +6,7 @@
 namespace he4 {
 namespace regfft {
 
-// complex type of a real type
-template <typename T>
-struct Cx;
-template <>
-struct Cx<double> {
-  using type = double2;
-};
-template <>
-struct Cx<float> {
-  using type = float2;
-};
-
+// real type of a complex type
 template <typename C2>
 struct Re;
 template <>

@@ -10,8 +10,8 @@
 //          psix and of the force term),
 //   D+m  = D widened by the stencil half width (the support of hpsix).
 // The box is found on the device every evaluation; the previous box is
-// cleared, so denx, psix and hpsix stay zero outside the current one
-// and the full-grid FFT of denx sees exact zeros there.  When D+2m would
+// cleared, so denx, psix and hpsix stay zero outside the current one, and
+// the x/y transform of denx is done on the box's planes (fft_r2c_box).  When D+2m would
 // reach a face of the grid (periodic wrap of the stencils, boundary rows the
 // ironing leaves untouched) every box kernel covers the whole grid instead,
 // which is the reference's computation as it stands.

@@ -1,8 +1,10 @@
 // reduce.cuh -- deterministic FP64 block reductions.
 //
-// Every reduction is a fixed tree: warp shuffles, then one warp over the
-// per-warp sums, then a single CTA over the per-block partials in index
-// order.  Results therefore do not depend on scheduling.
+// Every reduction is a fixed tree: warp shuffles, then one warp over the per-warp
+// sums, then the per-block partials in a fixed assignment of indices to threads:
+// by the block that finishes last (grid_sums_last), or for the partials of a grid
+// kernel by up to 32 further blocks (finalize_sums).  Results therefore do not
+// depend on scheduling.
 #pragma once
 #include "common.cuh"
 
