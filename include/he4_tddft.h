@@ -61,8 +61,10 @@ enum {
  * HE4_PREC_FP64: everything in FP64 (the reference's arithmetic).
  * HE4_PREC_FP32CONV: the half spectra of the convolution FFTs, their
  *   twiddles, the k-space kernels (wcgk, fvlj4, kalfs, Vq) and the derivative
- *   symbol are FP32; real grids, the wavefunction update, the reductions and
- *   the particle integration stay FP64.  Needs every axis length to be a
+ *   symbol are FP32; the wavefunction update, the reductions, the particle
+ *   integration and the real grids that calls return or energies sum stay FP64
+ *   (a time step's own intermediate grids are float, pot4 and den FP64).
+ *   Needs every axis length to be a
  *   power of two in [16, 256]; otherwise he4_create returns
  *   HE4_E_UNSUPPORTED. */
 enum { HE4_PREC_FP64 = 0, HE4_PREC_FP32CONV = 1 };
