@@ -1,9 +1,9 @@
 """he4_energy's convolution energies, summed over k (csrc/fft_mix.cuh
 k_mix_zenergy), against the sums over the grid of the fields they stand for:
 every z length with a two-step transform, whose CTAs have 48 to 216 threads at work,
-few of them a multiple of 32, on
-x and y axes that leave tiles with a remainder.  Both are sums of a few thousand
-products in FP64: they agree to 1e-12 of the sum of the magnitudes."""
+few of them a multiple of 32, on x and y axes that leave tiles with a remainder.
+Both are sums of a few thousand products in FP64: they agree to 1e-12 of the sum of
+the magnitudes."""
 import numpy as np
 import pytest
 
